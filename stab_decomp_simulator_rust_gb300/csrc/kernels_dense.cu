@@ -21,6 +21,10 @@ namespace {
 using dev::FULL;
 
 constexpr int DWARPS = 4;
+// Exponents of restored terms are any 32-bit numbers: beyond ±kMaxExponent the
+// integers are refused, and twice that is where they are cut off, so that no sum or
+// difference of them overflows (the weights index shared memory).
+constexpr int kMaxExponent = 1 << 20;
 
 template <typename Desc>
 __device__ __forceinline__ const Desc& owner_of(const Desc* descs, int num, int64_t i, int64_t Desc::*begin) {
@@ -135,7 +139,8 @@ __global__ void __launch_bounds__(DWARPS * 32) dense_terms_kernel(const DenseDes
             o->piv = piv;
             o->rhs = rhs;
             o->k0 = (tv.phase[term] + tv.coef_k[term]) & 7;
-            d.kr[term] = make_int2(o->k0, empty ? INT_MIN : __popc(v) + tv.coef_r[term]);
+            d.kr[term] = make_int2(o->k0, empty ? INT_MIN
+                                                : __popc(v) + min(max(tv.coef_r[term], -2 * kMaxExponent), 2 * kMaxExponent));
         }
     }
 }
@@ -175,7 +180,7 @@ __global__ void __launch_bounds__(OTHREADS) dense_order_kernel(const DenseDesc* 
         const int2 kr = i < chi ? d.kr[i] : make_int2(0, INT_MIN);
         if (kr.y == INT_MIN) return -1;
         w = rmax - kr.y;
-        return w > 46 ? -2 : ((kr.x & 1) * 2 + (w & 1)) * 32 + (31 - (w >> 1));
+        return w > 46 || abs(kr.y) > kMaxExponent ? -2 : ((kr.x & 1) * 2 + (w & 1)) * 32 + (31 - (w >> 1));
     };
     unsigned mine = 0;
     const int rounds = (chi + OTHREADS - 1) / OTHREADS;
