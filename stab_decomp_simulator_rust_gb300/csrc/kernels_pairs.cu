@@ -1209,6 +1209,7 @@ __device__ __forceinline__ void load_form(const unsigned char* forms, int64_t te
 // add per term took a quarter of a pair's time; both precisions use this.
 template <int NG>
 struct IntAcc {
+    static constexpr int kUp = 22;  // bits left below a chunk's first term
     long long a[NG][2];
     int base[NG];
     __device__ __forceinline__ void reset() {
@@ -1222,7 +1223,8 @@ struct IntAcc {
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             if (a[g][c] == 0) continue;
-            const double val = (double)a[g][c] * pow2i(-base[g]);
+            // (two exact products: 2^-base alone is below the normal numbers for terms of 2^-1000)
+            const double val = (double)a[g][c] * 0x1p-22 * pow2i(kUp - base[g]);
             double s, err;
             two_sum_d(pp[2 * c], val, s, err);
             pp[2 * c] = s;
@@ -1232,12 +1234,12 @@ struct IntAcc {
         base[g] = INT_MIN;
     }
     __device__ __forceinline__ void add(int g, int cls, int sgn, int e, double* pp) {
-        if (base[g] == INT_MIN) base[g] = e + 22;
+        if (base[g] == INT_MIN) base[g] = e + kUp;
         int sh = base[g] - e;
-        if ((unsigned)sh > 44u) {
+        if ((unsigned)sh > 2u * kUp) {
             flush(g, pp);
-            base[g] = e + 22;
-            sh = 22;
+            base[g] = e + kUp;
+            sh = kUp;
         }
         const long long t = (long long)sgn << sh;
         a[g][0] += cls ? 0 : t;

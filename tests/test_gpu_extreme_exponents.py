@@ -26,3 +26,29 @@ def test_vector_with_exponents_that_overflow_their_difference(gpu_pkg, low, high
     want = gpu_pkg.QuantumState.from_terms(dict(keep, coef_r=keep["coef_r"] - np.int32(low))).to_statevector()
     want = want * 2.0 ** (-low / 2)
     np.testing.assert_allclose(got, want, rtol=0, atol=1e-13 * np.abs(want).max())
+
+
+def noalloc(st, p):
+    import ctypes as C
+    from stab_decomp_simulator_rust_gb300 import _ffi
+    out = C.c_double()
+    a = p.abi()
+    _ffi.check(_ffi.load().nsg_exp_value_noalloc(st._h, C.byref(a), C.byref(out)))
+    return out.value
+
+
+# summed a pair per lane, and (more than 32 qubits left over) a pair per warp
+@pytest.mark.parametrize("n,t,terms", [(34, 20, None), (40, 36, 400)])
+@pytest.mark.parametrize("shift", [-960, 960, 986])
+def test_values_near_the_ends_of_the_exponents(gpu_pkg, n, t, terms, shift):
+    """Pair terms down to 2^-1019 and up to 2^960: the values of the state without the shift, scaled."""
+    d = with_exponents(gpu_pkg, n, t, 5600 + n, lambda r: r + shift)
+    pick = np.sort(np.random.default_rng(n).permutation(len(d["phase"]))[:terms])
+    d = {k: v[pick] if isinstance(v, np.ndarray) and k != "global_factor" else v for k, v in d.items()}
+    st = gpu_pkg.QuantumState.from_terms(d)
+    base = gpu_pkg.QuantumState.from_terms(dict(d, coef_r=d["coef_r"] - np.int32(shift)))
+    ps = [gpu_pkg.PauliString.identity()] + [gpu_pkg.PauliString.sparse([3], [q]) for q in range(0, n, 7)]
+    want = [noalloc(base, p) for p in ps]
+    scale = 2.0 ** -shift
+    np.testing.assert_allclose(st.exp_values(ps) / scale, want, rtol=0, atol=1e-12 * want[0])
+    np.testing.assert_allclose(st.exp_values(ps, gpu_pkg.PRECISION_MIXED) / scale, want, rtol=0, atol=1e-12 * want[0])
