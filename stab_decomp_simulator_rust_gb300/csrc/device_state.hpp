@@ -160,14 +160,15 @@ cudaError_t launch_pauli_frames(const TermsView& t, const DevPauli* d_paulis, in
                                 uint64_t* x_out, uint8_t* k_out, cudaStream_t st);
 
 // ---- reduction by common stabilizers (kernels_reduce.cu, common_stabilizers.hpp)
-constexpr int kMaxBadTerms = 15;  // terms reported by one reduction that its generators do not fit
+constexpr int kMaxBadTerms = 15;    // terms reported by one reduction that its generators do not fit
+constexpr int kMaxExtraTerms = 32;  // terms that a search for the generators has to sample
 
 // A state whose common stabilizers are looked for: its terms (n ≤ 64, χ ≥ 1)
 // and terms that have to be among the sampled ones.
 struct CommonDesc {
     TermsView tv;
     int nextra = 0;
-    int64_t extra[32];
+    int64_t extra[kMaxExtraTerms];
 };
 struct CommonOut {  // generators i^k X(x) Z(z), and the sampled terms' number and Σ|v|
     int count, sampled, vsum;
