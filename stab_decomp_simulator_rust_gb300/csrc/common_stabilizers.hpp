@@ -40,16 +40,19 @@ inline void transpose64(uint64_t (&a)[64]) {
         }
 }
 
-// Generators of a group of stabilizers common to all terms of a state.
+// Independent generators of a group of stabilizers common to all terms of a
+// state: at most as many as qubits.
 struct CommonGroup {
     std::vector<HPauli> gens;
     double mean_v = -1.0;  // mean |v| of the sampled terms (for a choice of kernels only)
 
     // Conjugation by Clifford gates, all generators at once: bit i of X[q], Z[q]
     // is generator i's at qubit q, of R its sign as a product of I, X, Y, Z
-    // (i^k X(x) Z(z) has k = #Y + 2·sign).
-    void apply(const std::vector<uint32_t>& ops) {
-        if (gens.empty() || gens.size() > 64) return;
+    // (i^k X(x) Z(z) has k = #Y + 2·sign).  False: more generators than a word has
+    // bits, which stay as they are (nothing is known then).
+    bool apply(const std::vector<uint32_t>& ops) {
+        if (gens.empty()) return true;
+        if (gens.size() > 64) return false;
         uint64_t X[64] = {}, Z[64] = {}, R = 0;
         for (size_t i = 0; i < gens.size(); i++) {
             X[i] = gens[i].x;
@@ -97,20 +100,12 @@ struct CommonGroup {
             gens[i].z = Z[i];
             gens[i].k = (__builtin_popcountll(X[i] & Z[i]) + 2 * (int)((R >> i) & 1)) & 3;
         }
+        return true;
     }
     // The group after every term was projected on Z_q = (-1)^outcome (terms that
     // it annihilates left the state): the elements that commute with Z_q, and Z_q.
-    void project(int q, bool outcome) {
-        std::vector<HPauli> out;
-        const HPauli* pivot = nullptr;
-        for (const HPauli& g : gens) {
-            if (!((g.x >> q) & 1)) out.push_back(g);
-            else if (!pivot) pivot = &g;
-            else out.push_back(g * *pivot);
-        }
-        out.push_back({0, 1ull << q, outcome ? 2 : 0});
-        gens = std::move(out);
-    }
+    // False if -Z_q is one of them: no term is left, and nothing is known.
+    bool project(int q, bool outcome);
     // The group after qubit q (in |0⟩ in every term) was removed; false if Z_q
     // is not among the elements (then nothing is known).
     bool discard(int q);
@@ -221,6 +216,29 @@ inline bool Reduction::map(const DevPauli& p, DevPauli& out) const {
         if (parity64(z & ax[q])) out.pz |= 1ull << q;
     out.ny = (p.ny + 2 * parity64(x0 & p.pz) - r.k + 2 * parity64(z & g.x)) & 3;
     out.pad = 0;
+    return true;
+}
+
+inline bool CommonGroup::project(int q, bool outcome) {
+    const HPauli zq{0, 1ull << q, outcome ? 2 : 0};
+    std::vector<HPauli> out;
+    const HPauli* pivot = nullptr;
+    for (const HPauli& g : gens) {
+        if (!((g.x >> q) & 1)) out.push_back(g);
+        else if (!pivot) pivot = &g;
+        else out.push_back(g * *pivot);
+    }
+    if (!pivot) {  // Z_q commutes with every element: it may be one, up to its sign
+        std::vector<HPauli> rows = gens;
+        const size_t nx = reduce_rows(rows, 0, ~0ull, true).size();
+        const std::vector<int> pz = reduce_rows(rows, nx, ~0ull, false);
+        HPauli rest = zq;
+        for (size_t j = 0; j < pz.size(); j++)
+            if ((rest.z >> pz[j]) & 1) rest = rest * rows[nx + j];
+        if (rest.z == 0) return !(rest.k & 2);
+    }
+    out.push_back(zq);
+    gens = std::move(out);
     return true;
 }
 
