@@ -210,6 +210,7 @@ cudaError_t launch_reduce_terms(const ReduceDesc* descs, int num, int64_t total,
 // ---- amplitudes as exact integers (kernels_dense.cu), n ≤ 26 -------------------
 constexpr int kDenseMaxQubits = 26;  // 2^26 points of 16 bytes: 1 GB
 constexpr int kDensePlanes = 24;     // bits of a coordinate, with its sign
+constexpr int64_t kDenseMaxTerms = (int64_t)1 << (kDensePlanes - 1);  // each counts 1 at least: as many never fit
 constexpr int kDenseKeys = 128;      // (group of four, weight 2^31 .. 2^0) of a term
 
 // One term as a quadratic form (dense_terms_kernel).
