@@ -247,10 +247,14 @@ nsg_status nsg_zero_screen_circuit(uint32_t num_qubits, const nsg_gate* gates, s
                                    const nsg_pauli* paulis, size_t num_paulis, uint8_t* zero);
 
 /* Tiling of the direct (uncaptured) pair sums of this process: kets per
- * chunk and tasks per resident warp of the persistent pair launch; 0 takes
+ * chunk and tasks per resident warp of the persistent pair launches; 0 takes
  * the tuned choice of the workload class if a plan tuned one, else the
- * default (32 and 64).  Results do not depend on it beyond FP rounding of the
- * partial sums (no reference counterpart). */
+ * default: 32 kets, or as few as 2 where a launch has too few pairs for that
+ * many, and 64 tasks.  Launches over reduced terms as quadratic forms are not
+ * tuned and default to 12 tasks; their chunks have at most 64 kets, and exactly
+ * 32 where a lane holds a pair (up to 32 qubits left).  Sums that come from
+ * amplitudes have no pairs to tile.  Results do not depend on it beyond FP
+ * rounding of the partial sums (no reference counterpart). */
 nsg_status nsg_set_pair_tiling(int32_t chunk, int32_t tasks_per_warp);
 
 /* ⟨P⟩ for callers that cannot allocate device memory at call time — a

@@ -391,7 +391,7 @@ def compile_keep(num_qubits: int, gates) -> np.ndarray:
 
 
 def set_pair_tiling(chunk: int = 0, tasks_per_warp: int = 0) -> None:
-    """Tiling of direct pair sums in this process (0 = default)."""
+    """Kets per chunk and tasks per resident warp of direct pair sums in this process (0 = default)."""
     check(_ffi.load().nsg_set_pair_tiling(chunk, tasks_per_warp))
 
 
