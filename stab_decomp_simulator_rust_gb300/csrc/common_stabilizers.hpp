@@ -44,13 +44,19 @@ inline void transpose64(uint64_t (&a)[64]) {
 // state: at most as many as qubits.
 struct CommonGroup {
     std::vector<HPauli> gens;
-    double mean_v = -1.0;  // mean |v| of the sampled terms (for a choice of kernels only)
+    // Mean |v| of sampled terms, for a choice of kernels only, and the H gates and
+    // projections since they were sampled: each changes a term's |v| by one at most.
+    double mean_v = -1.0;
+    int v_changes = 0;
+    void v_changed() { v_changes = v_changes < 128 ? v_changes + 1 : v_changes; }
 
     // Conjugation by Clifford gates, all generators at once: bit i of X[q], Z[q]
     // is generator i's at qubit q, of R its sign as a product of I, X, Y, Z
     // (i^k X(x) Z(z) has k = #Y + 2·sign).  False: more generators than a word has
     // bits, which stay as they are (nothing is known then).
     bool apply(const std::vector<uint32_t>& ops) {
+        for (uint32_t c : ops)
+            if ((c & 0xff) == P_H) v_changed();
         if (gens.empty()) return true;
         if (gens.size() > 64) return false;
         uint64_t X[64] = {}, Z[64] = {}, R = 0;
@@ -65,7 +71,7 @@ struct CommonGroup {
         for (uint32_t c : ops) {
             const uint32_t op = c & 0xff, a = (c >> 8) & 0xff, b = (c >> 16) & 0xff;
             switch (op) {
-                case P_H:
+                case P_H:  // the only gate that changes v
                     R ^= X[a] & Z[a];
                     std::swap(X[a], Z[a]);
                     break;
@@ -220,6 +226,7 @@ inline bool Reduction::map(const DevPauli& p, DevPauli& out) const {
 }
 
 inline bool CommonGroup::project(int q, bool outcome) {
+    v_changed();
     const HPauli zq{0, 1ull << q, outcome ? 2 : 0};
     std::vector<HPauli> out;
     const HPauli* pivot = nullptr;
@@ -243,6 +250,7 @@ inline bool CommonGroup::project(int q, bool outcome) {
 }
 
 inline bool CommonGroup::discard(int q) {
+    v_changed();
     const uint64_t bit = 1ull << q;
     // bring Z_q to a row of its own: reduce on z with column q last, over the Z-type rows
     std::vector<HPauli> g = gens;

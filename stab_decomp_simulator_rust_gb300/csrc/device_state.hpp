@@ -160,7 +160,9 @@ cudaError_t launch_pauli_frames(const TermsView& t, const DevPauli* d_paulis, in
                                 uint64_t* x_out, uint8_t* k_out, cudaStream_t st);
 
 // ---- reduction by common stabilizers (kernels_reduce.cu, common_stabilizers.hpp)
-constexpr int kMaxBadTerms = 15;    // terms reported by one reduction that its generators do not fit
+constexpr int kMaxBadTerms = 14;    // terms reported by one reduction that its generators do not fit
+constexpr int kReduceFlags = 16;    // flag words of one reduction (ReduceDesc)
+constexpr int kSampledV = 64;       // about as many terms' |v| are summed
 constexpr int kMaxExtraTerms = 32;  // terms that a search for the generators has to sample
 
 // A state whose common stabilizers are looked for: its terms (n ≤ 64, χ ≥ 1)
@@ -195,7 +197,8 @@ constexpr size_t form_bytes(int n) { return sizeof(FormHeader) + (n <= 32 ? 2 * 
 
 // One state's reduction: rows[0 .. out.n) the logical X operators, rows[out.n ..
 // in.n) the generators; out (W = 1) receives the reduced terms, flag[0] the
-// number of terms that the generators do not fit, flag[1 ..] the first of them.
+// number of terms that the generators do not fit, flag[1 .. kMaxBadTerms] the first
+// of them, flag[kReduceFlags - 1] Σ|v'| of every v_stride-th reduced term.
 struct ReduceDesc {
     TermsView in, out;
     unsigned char* forms = nullptr;  // [chi][form_bytes(out.n)]
@@ -204,6 +207,7 @@ struct ReduceDesc {
     int rx = 0;
     int64_t term0 = 0;  // terms of the launch before this state's
     int* flag = nullptr;
+    uint32_t v_stride = 1;
 };
 cudaError_t launch_reduce_terms(const ReduceDesc* descs, int num, int64_t total, cudaStream_t st);
 

@@ -464,6 +464,7 @@ __global__ void __launch_bounds__(RWARPS * 32) reduce_terms_kernel(const ReduceD
         o.phase[term] = (uint8_t)(phase & 7);
         o.coef_k[term] = tv.coef_k[term];
         o.coef_r[term] = tv.coef_r[term];
+        if ((uint32_t)term % d.v_stride == 0) atomicAdd(&d.flag[kReduceFlags - 1], __popcll(v2));
         if (any_bad) {
             const int at = atomicAdd(&d.flag[0], 1);
             if (at < kMaxBadTerms) d.flag[1 + at] = (int)term;
