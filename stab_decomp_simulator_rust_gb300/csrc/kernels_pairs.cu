@@ -1173,28 +1173,27 @@ __global__ void __launch_bounds__(PWARPS * 32, MINB) pair_kernel(MultiLaunch p) 
 // dependent shuffles and ballots, with 32 warps per SM to hide them: 1.08 ns per
 // pair at n2 = 34, χ = 13,122, where the table kernel takes 1.94.  (Up to 32 qubits
 // the lane kernel below is the faster one.)
-template <typename Word>
 struct FormKet {
-    Word L0, L1, piv, rhs;
+    uint64_t L0, L1, piv, rhs;
     int r, coef_r, phase, coef_k;
 };
 
-template <typename Word, int RPL>
-__device__ __forceinline__ void load_form(const unsigned char* forms, int64_t term, int lane, Word (&J)[RPL],
-                                          Word (&R)[RPL], FormKet<Word>& k) {
-    constexpr int ROWS = 32 * RPL;
-    const unsigned char* fp = forms + (size_t)term * (sizeof(FormHeader) + 2 * ROWS * sizeof(Word));
-    const Word* rows = (const Word*)(fp + sizeof(FormHeader));
+// A term of 33 to 64 qubits: lane l holds rows l and 32 + l.
+__device__ __forceinline__ void load_form(const unsigned char* forms, int64_t term, int lane, uint64_t (&J)[2],
+                                          uint64_t (&R)[2], FormKet& k) {
+    constexpr int ROWS = 64;
+    const unsigned char* fp = forms + (size_t)term * (sizeof(FormHeader) + 2 * ROWS * sizeof(uint64_t));
+    const uint64_t* rows = (const uint64_t*)(fp + sizeof(FormHeader));
 #pragma unroll
-    for (int t = 0; t < RPL; t++) {
+    for (int t = 0; t < 2; t++) {
         J[t] = rows[32 * t + lane];
         R[t] = rows[ROWS + 32 * t + lane];
     }
     const FormHeader* h = (const FormHeader*)fp;
-    k.L0 = (Word)h->L0;
-    k.L1 = (Word)h->L1;
-    k.piv = (Word)h->piv;
-    k.rhs = (Word)h->rhs;
+    k.L0 = h->L0;
+    k.L1 = h->L1;
+    k.piv = h->piv;
+    k.rhs = h->rhs;
     k.r = h->r;
     k.coef_r = h->coef_r;
     const uint32_t pc = *(const uint32_t*)&h->phase;
@@ -1247,8 +1246,10 @@ struct IntAcc {
     }
 };
 
-template <typename Word, int RPL, int NG, int MINB>
+template <int NG, int MINB>
 __global__ void __launch_bounds__(PWARPS * 32, MINB) pair_form_kernel(MultiLaunch p) {
+    using Word = uint64_t;
+    constexpr int RPL = 2;  // row slots per lane
     const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int gwarp = blockIdx.x * PWARPS + wid;
     Word own[RPL];
@@ -1260,7 +1261,7 @@ __global__ void __launch_bounds__(PWARPS * 32, MINB) pair_form_kernel(MultiLaunc
     int64_t chi = 0, cur_i = -1;
     Word JA[RPL], RA[RPL], hA[NG], cA[NG];
     int kA[NG];
-    FormKet<Word> a;
+    FormKet a;
     int64_t task = gwarp;
     while (task < p.total_tasks) {
         if (ds < 0 || task >= p.task_begin[ds + 1]) {
@@ -1281,7 +1282,7 @@ __global__ void __launch_bounds__(PWARPS * 32, MINB) pair_form_kernel(MultiLaunc
             const int64_t j0 = max(i, kb * (int64_t)p.chunk), j1 = min((kb + 1) * (int64_t)p.chunk, chi);
             if (i != cur_i) {
                 cur_i = i;
-                load_form<Word, RPL>(d->forms, i, lane, JA, RA, a);
+                load_form(d->forms, i, lane, JA, RA, a);
 #pragma unroll
                 for (int g = 0; g < NG; g++) {
                     const int o = 32 * g + lane;
@@ -1293,19 +1294,19 @@ __global__ void __launch_bounds__(PWARPS * 32, MINB) pair_form_kernel(MultiLaunc
             }
             IntAcc<NG> acc;
             acc.reset();
-            const Word full = (n >= 8 * (int)sizeof(Word)) ? ~(Word)0 : (((Word)1 << n) - 1);
+            const Word full = n >= 64 ? ~(Word)0 : ((Word)1 << n) - 1;
             Word Jn[RPL], Rn[RPL];
-            FormKet<Word> bn;
-            load_form<Word, RPL>(d->forms, j0, lane, Jn, Rn, bn);
+            FormKet bn;
+            load_form(d->forms, j0, lane, Jn, Rn, bn);
             for (int64_t j = j0; j < j1; j++) {
                 Word J[RPL], RB[RPL];
-                const FormKet<Word> b = bn;
+                const FormKet b = bn;
 #pragma unroll
                 for (int k = 0; k < RPL; k++) {
                     J[k] = JA[k] ^ Jn[k];
                     RB[k] = Rn[k];
                 }
-                if (j + 1 < j1) load_form<Word, RPL>(d->forms, j + 1, lane, Jn, Rn, bn);  // in flight during this pair
+                if (j + 1 < j1) load_form(d->forms, j + 1, lane, Jn, Rn, bn);  // in flight during this pair
                 Word L0 = a.L0 ^ b.L0, hs = a.L1 ^ b.L1 ^ (a.L0 & ~b.L0);  // L_b - L_a mod 4
                 Word alive = full;
                 Word h[NG];
@@ -1320,7 +1321,7 @@ __global__ void __launch_bounds__(PWARPS * 32, MINB) pair_form_kernel(MultiLaunc
                 // the bra's constraints: z_k = R_k·z ⊕ rhs_k
                 Word m = a.piv;
                 while (m) {
-                    on_bit<Word, sizeof(Word) == 8>(m, [&](auto slot, int q) {
+                    on_bit<Word, true>(m, [&](auto slot, int q) {
                         constexpr int H = decltype(slot)::value;
                         const Word kb1 = (Word)(1u << q) << (32 * H);
                         m ^= kb1;
@@ -1362,7 +1363,7 @@ __global__ void __launch_bounds__(PWARPS * 32, MINB) pair_form_kernel(MultiLaunc
                             for (int g = 0; g < NG; g++) zero[g] |= c[g];
                             continue;
                         }
-                        on_bit<Word, sizeof(Word) == 8>(l, [&](auto slot, int q) {
+                        on_bit<Word, true>(l, [&](auto slot, int q) {
                             constexpr int H = decltype(slot)::value;
                             const Word kb1 = (Word)(1u << q) << (32 * H);
                             const Word lp = l ^ kb1;
@@ -1377,28 +1378,21 @@ __global__ void __launch_bounds__(PWARPS * 32, MINB) pair_form_kernel(MultiLaunc
                 }
                 int r = a.r + b.r;
                 Word IE = 0, IO = 0;
-                bool dead;
-                if constexpr (sizeof(Word) == 8) {
-                    dead = sum_out<Word, RPL, NG, true>(J, hs, L0, alive, IE, IO, r, h, ph, zero, own,
-                                                        ~(Word)0xffffffffu);
-                    if (!dead) {
-                        uint32_t J32[1] = {(uint32_t)J[0]};
-                        const uint32_t own32[1] = {(uint32_t)own[0]};
-                        uint32_t hs32 = (uint32_t)hs, L032 = (uint32_t)L0, alive32 = (uint32_t)alive, IE32 = 0, IO32 = 0;
-                        uint32_t h32[NG];
+                bool dead = sum_out<Word, RPL, NG, true>(J, hs, L0, alive, IE, IO, r, h, ph, zero, own, ~(Word)0xffffffffu);
+                if (!dead) {
+                    uint32_t J32[1] = {(uint32_t)J[0]};
+                    const uint32_t own32[1] = {(uint32_t)own[0]};
+                    uint32_t hs32 = (uint32_t)hs, L032 = (uint32_t)L0, alive32 = (uint32_t)alive, IE32 = 0, IO32 = 0;
+                    uint32_t h32[NG];
 #pragma unroll
-                        for (int g = 0; g < NG; g++) h32[g] = (uint32_t)h[g];
-                        dead = sum_out<uint32_t, 1, NG, false>(J32, hs32, L032, alive32, IE32, IO32, r, h32, ph, zero,
-                                                               own32, ~0u);
-                        const Word hi = ~(Word)0xffffffffu;
-                        hs = (hs & hi) | hs32;
+                    for (int g = 0; g < NG; g++) h32[g] = (uint32_t)h[g];
+                    dead = sum_out<uint32_t, 1, NG, false>(J32, hs32, L032, alive32, IE32, IO32, r, h32, ph, zero, own32, ~0u);
+                    const Word hi = ~(Word)0xffffffffu;
+                    hs = (hs & hi) | hs32;
 #pragma unroll
-                        for (int g = 0; g < NG; g++) h[g] = (h[g] & hi) | h32[g];
-                        IE |= IE32;
-                        IO |= IO32;
-                    }
-                } else {
-                    dead = sum_out<Word, RPL, NG, false>(J, hs, L0, alive, IE, IO, r, h, ph, zero, own, ~(Word)0);
+                    for (int g = 0; g < NG; g++) h[g] = (h[g] & hi) | h32[g];
+                    IE |= IE32;
+                    IO |= IO32;
                 }
                 if (dead) continue;
                 r -= 2 * popc<Word>(IE) + popc<Word>(IO);
@@ -2368,10 +2362,10 @@ cudaError_t launch_pairs_form(const MultiLaunch& m, cudaStream_t st) {
     if (m.total_tasks == 0) return cudaSuccess;
     const int ng = (m.nobs_max + 31) / 32;
     const dim3 grid(m.blocks), block(PWARPS * 32);
-    if (ng <= 1) pair_form_kernel<uint64_t, 2, 1, form_minb(1)><<<grid, block, 0, st>>>(m);
-    else if (ng <= 2) pair_form_kernel<uint64_t, 2, 2, form_minb(2)><<<grid, block, 0, st>>>(m);
-    else if (ng <= 4) pair_form_kernel<uint64_t, 2, 4, form_minb(4)><<<grid, block, 0, st>>>(m);
-    else if (ng <= 8) pair_form_kernel<uint64_t, 2, 8, form_minb(8)><<<grid, block, 0, st>>>(m);
+    if (ng <= 1) pair_form_kernel<1, form_minb(1)><<<grid, block, 0, st>>>(m);
+    else if (ng <= 2) pair_form_kernel<2, form_minb(2)><<<grid, block, 0, st>>>(m);
+    else if (ng <= 4) pair_form_kernel<4, form_minb(4)><<<grid, block, 0, st>>>(m);
+    else if (ng <= 8) pair_form_kernel<8, form_minb(8)><<<grid, block, 0, st>>>(m);
     else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
