@@ -638,16 +638,11 @@ __global__ void __launch_bounds__(VTHREADS) dense_weights_kernel(const int4* __r
 __global__ void __launch_bounds__(VTHREADS) dense_vector_kernel(const int4* __restrict__ psi, const DenseInfo* info, int n,
                                                                 double gf_re, double gf_im, double2* __restrict__ out) {
     if (!info->ok) return;
-    const double r2 = 0.70710678118654752440;
-    const int R = info->rmax;
-    // 2^{-R/2}: an exact power of two, times 1/√2 for odd R
-    const double p = ldexp((R & 1) ? r2 : 1.0, -((R - (R & 1)) / 2));
-    const double sr = gf_re * p, si = gf_im * p;
+    const dev::AmplitudeScale amplitude(info->rmax, gf_re, gf_im);
     const uint64_t pts = (uint64_t)1 << n;
     for (uint64_t x = (uint64_t)blockIdx.x * VTHREADS + threadIdx.x; x < pts; x += (uint64_t)gridDim.x * VTHREADS) {
         const int4 c = psi[x];  // (c0, c2, c1, c3)
-        const double re = (double)c.x + (double)(c.z - c.w) * r2, im = (double)c.y + (double)(c.z + c.w) * r2;
-        out[x] = make_double2(re * sr - im * si, re * si + im * sr);
+        out[x] = amplitude(c.x, c.z, c.y, c.w);
     }
 }
 

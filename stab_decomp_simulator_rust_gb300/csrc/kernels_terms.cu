@@ -7,6 +7,8 @@
 // read each op from one broadcast load.
 #include <cuda_runtime.h>
 
+#include <climits>
+
 #include "device_state.hpp"
 #include "warp_chform.cuh"
 
@@ -694,18 +696,49 @@ __global__ void pack_kernel(TermsView tv, const uint8_t* G, const uint8_t* F, co
     }
 }
 
-// ---- dense statevector (n ≤ 28; tests and to_statevector) -------------------
+// ---- dense statevector (n ≤ 28), one point per thread -----------------------------
 // ⟨x|U_C U_H|s⟩ = i^{Σ_{p∈x}γ_p}·(-1)^{Σ_{p<q∈x} M_p·F_q + u·m + Σ_{j∈v} u_j s_j}·2^{-|v|/2}
 // with u = xF, m = xM, nonzero iff u_j = s_j for all j ∉ v.  Same value as
 // amplitude_at_computational_basis (form/amplitude.rs:28-44).
-__global__ void statevector_kernel(TermsView tv, double gf_re, double gf_im, double* __restrict__ out) {
+// The terms are summed as integers c0 + c1 ω + c2 ω² + c3 ω³ in units of 2^{-R/2} (R
+// the largest exponent), as the amplitude kernels do, where these stay below 2^52;
+// else in FP64.  One launch and no scratch: for few terms (api.cu, vector_direct).
+constexpr int VEC_THREADS = 256;
+
+__global__ void __launch_bounds__(VEC_THREADS) statevector_kernel(TermsView tv, double gf_re, double gf_im,
+                                                                  double2* __restrict__ out) {
+    __shared__ int ends[2];  // largest and smallest exponent
+    if (threadIdx.x == 0) {
+        ends[0] = INT_MIN;
+        ends[1] = INT_MAX;
+    }
+    __syncthreads();
+    constexpr int kMaxExponent = 1 << 20;  // (restored terms have any: differences stay 32-bit numbers)
+    int most = INT_MIN, least = INT_MAX;
+    for (int64_t term = threadIdx.x; term < tv.chi; term += VEC_THREADS) {
+        const int r = __popcll(tv.V[term * tv.W]) + min(max(tv.coef_r[term], -2 * kMaxExponent), 2 * kMaxExponent);
+        most = max(most, r);
+        least = min(least, r);
+    }
+    most = __reduce_max_sync(dev::FULL, most);
+    least = __reduce_min_sync(dev::FULL, least);
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&ends[0], most);
+        atomicMin(&ends[1], least);
+    }
+    __syncthreads();
+    const int R = ends[0];
+    const bool exact = tv.chi > 0 && (R - ends[1] + 1) / 2 + (64 - __clzll(tv.chi)) <= 52 && abs(R) < kMaxExponent &&
+                       abs(ends[1]) < kMaxExponent;
     const int n = tv.n;
     const int64_t dim = (int64_t)1 << n;
     const double r2 = 0.70710678118654752440;
     const double cr[8] = {1, r2, 0, -r2, -1, -r2, 0, r2};
     const double ci[8] = {0, r2, 1, r2, 0, -r2, -1, -r2};
-    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < dim; x += (int64_t)gridDim.x * blockDim.x) {
+    const dev::AmplitudeScale amplitude(exact ? R : 0, gf_re, gf_im);
+    for (int64_t x = (int64_t)blockIdx.x * VEC_THREADS + threadIdx.x; x < dim; x += (int64_t)gridDim.x * VEC_THREADS) {
         double ar = 0.0, ai = 0.0;
+        long long c0 = 0, c1 = 0, c2 = 0, c3 = 0;
         for (int64_t term = 0; term < tv.chi; term++) {
             const uint64_t* F = tv.F + (size_t)term * tv.R * tv.W;
             const uint64_t* M = tv.M + (size_t)term * tv.R * tv.W;
@@ -726,12 +759,28 @@ __global__ void statevector_kernel(TermsView tv, double gf_re, double gf_im, dou
             cnt += __popcll(u & m) + __popcll(u & v & s);
             int k = (tv.phase[term] + 2 * gsum + 4 * (cnt & 1) + tv.coef_k[term]) & 7;
             int rr = __popcll(v) + tv.coef_r[term];
+            if (exact) {  // ω^k·2^{w/2}; √2 = ω + ω^{-1}
+                const int w = R - rr;
+                auto add = [&](int j) {
+                    const long long t = (j & 4) ? -(1LL << (w >> 1)) : 1LL << (w >> 1);
+                    c0 += (j & 3) == 0 ? t : 0;
+                    c1 += (j & 3) == 1 ? t : 0;
+                    c2 += (j & 3) == 2 ? t : 0;
+                    c3 += (j & 3) == 3 ? t : 0;
+                };
+                if (w & 1) {
+                    add(k + 1);
+                    add(k + 7);
+                } else {
+                    add(k);
+                }
+                continue;
+            }
             double mag = exp2(-0.5 * (double)rr);
             ar += mag * cr[k];
             ai += mag * ci[k];
         }
-        out[2 * x] = ar * gf_re - ai * gf_im;
-        out[2 * x + 1] = ar * gf_im + ai * gf_re;
+        out[x] = exact ? amplitude(c0, c1, c2, c3) : make_double2(ar * gf_re - ai * gf_im, ar * gf_im + ai * gf_re);
     }
 }
 
@@ -904,7 +953,7 @@ cudaError_t launch_kron(TermsView A, TermsView B, TermsView O, cudaStream_t st) 
 cudaError_t launch_statevector(const TermsView& t, double gf_re, double gf_im, double* out, cudaStream_t st) {
     int64_t dim = (int64_t)1 << t.n;
     int blocks = (int)std::min<int64_t>((dim + 255) / 256, 65535);
-    statevector_kernel<<<blocks, 256, 0, st>>>(t, gf_re, gf_im, out);
+    statevector_kernel<<<blocks, VEC_THREADS, 0, st>>>(t, gf_re, gf_im, (double2*)out);
     return cudaGetLastError();
 }
 

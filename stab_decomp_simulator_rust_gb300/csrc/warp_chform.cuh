@@ -228,6 +228,24 @@ struct BV {
     }
 };
 
+// g·2^{-R/2}·(c0 + c1 ω + c2 ω² + c3 ω³), ω = e^{iπ/4}, of exact integers: what both
+// state vector kernels end with.
+struct AmplitudeScale {
+    double re, im;  // g·2^{-R/2}
+    __device__ __forceinline__ AmplitudeScale(int R, double gf_re, double gf_im) {
+        // an exact power of two, times 1/√2 for odd R
+        const double p = ldexp((R & 1) ? 0.70710678118654752440 : 1.0, -((R - (R & 1)) / 2));
+        re = gf_re * p;
+        im = gf_im * p;
+    }
+    template <typename Int>
+    __device__ __forceinline__ double2 operator()(Int c0, Int c1, Int c2, Int c3) const {
+        const double r2 = 0.70710678118654752440;
+        const double a = (double)c0 + (double)(c1 - c3) * r2, b = (double)c2 + (double)(c1 + c3) * r2;
+        return make_double2(a * re - b * im, a * im + b * re);
+    }
+};
+
 // A row slot known when the code is compiled.
 template <int K>
 struct Slot {
