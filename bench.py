@@ -70,10 +70,8 @@ METRIC = "Pauli ⟨P⟩/s and CH inner products/s, mixed+batched vs plain FP64 @
 UNIT = "<P>/s"
 WORKLOAD = "512 circuits, n~U[8,64], t~U[4,32], 20n {H,S,CX}, 16 dense Paulis each (seed 4)"
 
-# DRAM bytes (read + write) of a pair launch of the kernel that the roofline
-# times, from one ncu capture (64 observables, 8,748 reduced terms of 32 qubits):
-# 2.1 GB/s over 16.3 ms.  The terms' forms (0.3 KB each) stay in L2.
-PAIR_TRAFFIC_BYTES = 34_300_000
+# Kernels of a pair launch as nsg_profile_launch numbers them.
+PAIR_KERNELS = {0: "pair_kernel (term tables)", 1: "pair_form_kernel", 2: "pair_lane_kernel"}
 
 
 def dist_env():
@@ -270,16 +268,18 @@ def _int_peak(L):
 
 
 def _pair_profile(L, fn):
-    """Runs fn() with pair-kernel profiling on: (ms summed over launches, launches, pairs)."""
+    """Runs fn() with pair-kernel profiling on: (ms summed over launches, launches, pairs, and of the
+    launch with the most pairs its kernel and the qubits of its terms)."""
     import ctypes as C
     from stab_decomp_simulator_rust_gb300 import _ffi
     _ffi.check(L.nsg_profile_enable(1))
     _ffi.check(L.nsg_profile_read(None, None, None))
     fn()
-    ms, nl, pr = C.c_double(), C.c_uint64(), C.c_uint64()
+    ms, nl, pr, kernel, width = C.c_double(), C.c_uint64(), C.c_uint64(), C.c_int32(), C.c_int32()
+    _ffi.check(L.nsg_profile_launch(C.byref(kernel), C.byref(width)))
     _ffi.check(L.nsg_profile_read(C.byref(ms), C.byref(nl), C.byref(pr)))
     _ffi.check(L.nsg_profile_enable(0))
-    return ms.value, nl.value, pr.value
+    return ms.value, nl.value, pr.value, PAIR_KERNELS.get(kernel.value), width.value
 
 
 def _count_launches(torch, make):
@@ -508,30 +508,27 @@ def run_ours(args):
 
     # ---- roofline of the pair kernel: the direct call on one state, its launches event-timed
     launches = _count_launches(torch, lambda: BatchPlan(states, plists, PRECISION_MIXED).run)
-    step_ms, step_launches, step_pairs = _pair_profile(L, lambda: exp_values_multi(states, plists, PRECISION_MIXED))
-    pk_ms, pk_launches, pk_pairs, pk_state = 0.0, 0, 0, -1
-    for i in sorted(rest, key=lambda i: -pairs[i]):
+    step_ms, step_launches, step_pairs, _, _ = _pair_profile(L, lambda: exp_values_multi(states, plists, PRECISION_MIXED))
+    roofline = None
+    for i in sorted(rest, key=lambda i: -pairs[i]):  # the state with the most pairs left to sum, if any has some
         states[i].exp_values(plists[i])
-        pk_ms, pk_launches, pk_pairs = _pair_profile(L, lambda: states[i].exp_values(plists[i]))
-        if pk_pairs:
-            pk_state = i
-            break
-    word_peak = _int_peak(L)
-    t_of = int(np.isin(circuits[pk_state][1][:, 0], (W.OP["T"], W.OP["TDG"])).sum()) if pk_state >= 0 else 0
-    width = min(ns[pk_state], t_of)
-    # w(w-1)/2 row updates of a pair, each one word of J and one of the observables' bits,
-    # two XORs a word: as many 64-bit word operations (2 int32 operations) as words
-    ops = float(pk_pairs) * width * (width - 1)
-    achieved = ops / (pk_ms * 1e-3) if pk_ms else 0.0
-    roofline = {"bound": "int", "achieved": achieved / 1e12, "peak": word_peak / 1e12, "unit": "Tword-ops/s",
-                "frac": achieved / word_peak, "traffic": PAIR_TRAFFIC_BYTES,
-                "traffic_unit": "DRAM bytes of one launch over 8,748 reduced terms of 32 qubits, 64 observables (ncu)",
-                "kernel": "pair_lane_kernel on the state with the most pairs left to sum",
-                "peak_source": "measured on this GPU: LOP3 chains on every SM (nsg_probe_int_ops), "
-                               "a 64-bit word = 2 int32 logic ops",
-                "algorithmic_unit": "w(w-1) word-ops per term pair, w = min(n, t)", "width": width, "t": t_of,
-                "pair_kernel_ms": pk_ms, "launches": pk_launches, "pairs": pk_pairs,
-                "pair_kernels_ms_per_step": step_ms, "launches_per_step": step_launches, "pairs_per_step": step_pairs}
+        pk_ms, pk_launches, pk_pairs, pk_kernel, width = _pair_profile(L, lambda: states[i].exp_values(plists[i]))
+        if not pk_pairs:
+            continue
+        word_peak = _int_peak(L)
+        # w(w-1)/2 row updates of a pair, each one word of J and one of the observables' bits,
+        # two XORs a word: as many 64-bit word operations (2 int32 operations) as words
+        ops = float(pk_pairs) * width * (width - 1)
+        achieved = ops / (pk_ms * 1e-3)
+        roofline = {"bound": "int", "achieved": achieved / 1e12, "peak": word_peak / 1e12, "unit": "Tword-ops/s",
+                    "frac": achieved / word_peak, "kernel": pk_kernel + " on the state with the most pairs left to sum",
+                    "peak_source": "measured on this GPU: LOP3 chains on every SM (nsg_probe_int_ops), "
+                                   "a 64-bit word = 2 int32 logic ops",
+                    "algorithmic_unit": "w(w-1) word-ops per term pair, w = the qubits that its launch summed over",
+                    "width": width, "n": ns[i], "pair_kernel_ms": pk_ms, "launches": pk_launches, "pairs": pk_pairs,
+                    "pair_kernels_ms_per_step": step_ms, "launches_per_step": step_launches,
+                    "pairs_per_step": step_pairs}
+        break
 
     # ---- end to end from host buffers
     e2e_steps = max(1, min(3, args.steps))
@@ -564,8 +561,14 @@ def run_ours(args):
             "data": "synthetic (seeded generator)",
             "config": {"workload": WORKLOAD, "chi_min": min(chis), "chi_max": max(chis), "chi_sum": sum(chis),
                        "pairs_per_step": int(sum(pairs)), "observables_per_step": nobs,
-                       "l2": "inputs larger than L2 (term tables of 512 states)", "parallelism": f"replicas x{ws}"},
+                       "l2": "inputs larger than L2 (terms of 512 states, read by every step)",
+                       "parallelism": f"replicas x{ws}"},
+            "value_covers": {"observables": nobs, "exactly_zero": zero_screen["exact_zero"], "pairs_summed": step_pairs,
+                             "note": "per step; an observable that a stabilizer common to all terms of its state makes "
+                                     "zero is decided without pair sums, and every run checks the stabilizers on every "
+                                     "term: value counts those too, so it is no rate of pairs"},
             "inner_products_per_s": sum(p * len(ps) for p, ps in zip(pairs, plists)) / (ms_step * 1e-3),
+            "inner_products_note": "the pairs that the values stand for, summed or decided together",
             "path": "BatchPlan.run (nsg_plan_run: CUDA-graph replay), mixed precision",
             "plan": {"create_s": plan_s, "tiling": plan.tiling},
             "compile_s_512_circuits": compile_s,

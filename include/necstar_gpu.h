@@ -419,6 +419,10 @@ nsg_status nsg_export_terms(const nsg_state* state, uint8_t* G, uint8_t* F, uint
  * nsg_profile_read returns and resets the totals. */
 nsg_status nsg_profile_enable(int32_t enabled);
 nsg_status nsg_profile_read(double* pair_kernel_ms, uint64_t* launches, uint64_t* pairs);
+/* The launch with the most pairs since the last nsg_profile_read: its kernel (0:
+ * term tables; over quadratic forms 1: a pair per warp, 2: a pair per lane; -1: no
+ * launch) and the qubits of its terms (after the reduction by common stabilizers). */
+nsg_status nsg_profile_launch(int32_t* kernel, int32_t* width);
 
 /* Integer-pipe probe: runs a kernel of dependent-free 32-bit LOP3/XOR chains
  * on every SM for `iters` iterations and returns its duration and the number

@@ -89,6 +89,7 @@ def load(path: str | None = None):
     L.nsg_debug_chacha_block.argtypes = [vp, i32, vp]
     L.nsg_profile_enable.argtypes = [i32]
     L.nsg_profile_read.argtypes = [P(dbl), P(u64), P(u64)]
+    L.nsg_profile_launch.argtypes = [P(i32), P(i32)]
     L.nsg_probe_int_ops.argtypes = [u64, P(dbl), P(u64)]
     L.nsg_exp_value_counts.argtypes = [vp, P(PauliABI), sz, vp, P(dbl)]
     L.nsg_zero_screen.argtypes = [vp, P(PauliABI), sz, vp]
