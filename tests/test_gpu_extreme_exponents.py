@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from stab_decomp_simulator_rust_gb300 import workloads as W
+from term_sets import unrelated_terms
 
 pytestmark = pytest.mark.gpu
 
@@ -37,14 +38,16 @@ def noalloc(st, p):
     return out.value
 
 
-# summed a pair per lane, and (more than 32 qubits left over) a pair per warp
-@pytest.mark.parametrize("n,t,terms", [(34, 20, None), (40, 36, 400)])
+# summed a pair per lane, and (more than 32 qubits left) a pair per warp
+@pytest.mark.parametrize("n,t", [(34, 20), (40, 0)])
 @pytest.mark.parametrize("shift", [-960, 960, 986])
-def test_values_near_the_ends_of_the_exponents(gpu_pkg, n, t, terms, shift):
+def test_values_near_the_ends_of_the_exponents(gpu_pkg, n, t, shift):
     """Pair terms down to 2^-1019 and up to 2^960: the values of the state without the shift, scaled."""
-    d = with_exponents(gpu_pkg, n, t, 5600 + n, lambda r: r + shift)
-    pick = np.sort(np.random.default_rng(n).permutation(len(d["phase"]))[:terms])
-    d = {k: v[pick] if isinstance(v, np.ndarray) and k != "global_factor" else v for k, v in d.items()}
+    if t:
+        d = with_exponents(gpu_pkg, n, t, 5600 + n, lambda r: r + shift)
+    else:
+        d = unrelated_terms(gpu_pkg, n, 300, 5602)
+        d["coef_r"] = d["coef_r"] + np.int32(shift)
     st = gpu_pkg.QuantumState.from_terms(d)
     base = gpu_pkg.QuantumState.from_terms(dict(d, coef_r=d["coef_r"] - np.int32(shift)))
     ps = [gpu_pkg.PauliString.identity()] + [gpu_pkg.PauliString.sparse([3], [q]) for q in range(0, n, 7)]

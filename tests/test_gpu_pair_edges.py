@@ -9,24 +9,25 @@ import pytest
 
 from conftest import random_full_circuit
 from stab_decomp_simulator_rust_gb300 import workloads as W
+from term_sets import unrelated_terms
 from test_gpu_reduction import noalloc, observables
 
 pytestmark = pytest.mark.gpu
 
 
 # up to 32 qubits left (a pair per lane), and more (a pair per warp); the integers hold 44 powers of two
-@pytest.mark.parametrize("n,t,terms", [(34, 20, None), (40, 36, 400)])
+@pytest.mark.parametrize("n,extra", [(30, 10), (40, 0)])
 @pytest.mark.parametrize("spread", [86, 90, 130, 300])
-def test_exponents_beyond_a_chunk(gpu_pkg, n, t, terms, spread):
+def test_exponents_beyond_a_chunk(gpu_pkg, n, extra, spread):
     """Every third term 2^-(spread/2), every seventh 2^-spread: in turns, so that most chunks hold all three."""
-    gates = W.random_clifford_t_circuit(n, 20 * n, t, 6500 + n)
-    d = gpu_pkg.QuantumState.from_gates(n, gates).export_terms()
-    pick = np.sort(np.random.default_rng(n).permutation(len(d["phase"]))[:terms])
-    d = {k: v[pick] if isinstance(v, np.ndarray) and k != "global_factor" else v for k, v in d.items()}
+    d = unrelated_terms(gpu_pkg, n, 300, 6502)
     i = np.arange(len(d["phase"]))
     d["coef_r"] = (d["coef_r"] + spread * (i % 3 == 1) + 2 * spread * (i % 7 == 3)).astype(np.int32)
     st = gpu_pkg.QuantumState.from_terms(d)
-    ps = observables(gpu_pkg, n, gates, 3, 6)
+    if extra:
+        st = st.kron(gpu_pkg.QuantumState.from_gates(extra, np.zeros((0, 4), np.uint32)))
+    ps = [gpu_pkg.PauliString.sparse([3], [q]) for q in range(0, n + extra, 3)]
+    ps += [gpu_pkg.PauliString.dense(p) for p in W.random_dense_paulis(n + extra, 4, 6501)] + [gpu_pkg.PauliString.identity()]
     want = np.asarray([noalloc(st, p) for p in ps])
     for precision in (0, 1):
         np.testing.assert_allclose(st.exp_values(ps, precision), want, rtol=0, atol=1e-13 * max(1.0, want[-1]))
