@@ -40,5 +40,5 @@ def test_no_tables_beside_forms(gpu_pkg, plan):
     chi = int(chi)
     assert chi >= 15000 and abs(float(value) - 1.0) <= 1e-9
     # a reduced term takes at most 3 * 64 * 8 + 48 bytes, its form 1,072; tables
-    # and frames of 34 qubits and more would take 5,000 besides
+    # and frames would take 3,000 besides up to 32 qubits, 9,000 above
     assert int(used) <= chi * 2800, int(used) / chi

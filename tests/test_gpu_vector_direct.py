@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 def limit(n):
-    return int((42 if n <= 12 else 65) / max(0.6 + 0.13 * n, 2.3e-5 * 2 ** n))
+    return int((50 if n <= 12 else 65) / max(0.6 + 0.13 * n, 2.3e-5 * 2 ** n))
 
 
 @pytest.mark.parametrize("n", [1, 8, 12, 13, 16, 18, 20])
