@@ -210,7 +210,9 @@ nsg_status nsg_exp_value_batch(const nsg_state* state, const nsg_pauli* paulis,
                                size_t num_paulis, uint32_t precision, double* out);
 
 /* Batched form across states: observables paulis[pauli_offsets[c] ..
- * pauli_offsets[c+1]) on states[c], all in one persistent launch.  out has
+ * pauli_offsets[c+1]) on states[c], all states together: pairs from term tables
+ * (one launch for up to 32 qubits, one above), pairs of reduced terms as
+ * quadratic forms (likewise), and amplitudes of narrow states.  out has
  * pauli_offsets[num_states] entries.  No reference counterpart. */
 nsg_status nsg_exp_value_multi(const nsg_state* const* states, size_t num_states,
                                const nsg_pauli* paulis, const uint64_t* pauli_offsets,
@@ -279,12 +281,13 @@ nsg_status nsg_exp_value_noalloc(const nsg_state* state, const nsg_pauli* pauli,
  * to pinned host memory — captured once in a CUDA graph on the plan's own
  * stream.  nsg_plan_run replays it and writes pauli_offsets[num_states]
  * doubles to out.  Every run re-reads the states' current terms (a reduced
- * state's common stabilizers are checked on each of them).  Clifford gates applied in place (nsg_apply_gates) are seen by
- * the next run (states reduced by their common stabilizers are then summed
- * without the graph, which a second run on the same terms makes again); an
- * operation that changes a state's rank, width or global factor (projection,
- * discard, measurement) or frees it makes nsg_plan_run fail with
- * NSG_ERR_INVALID_ARGUMENT.  Creation picks, for each row width, the
+ * state's common stabilizers are checked on each of them).  Clifford gates
+ * applied in place (nsg_apply_gates) are seen by the next run (states reduced by
+ * their common stabilizers are then summed without the graph, which a second run
+ * on the same terms makes again; where making it fails, that run says so and the
+ * next one tries again).  An operation that changes a state's rank, width or
+ * global factor (projection, discard, measurement) or frees it makes nsg_plan_run
+ * fail with NSG_ERR_INVALID_ARGUMENT.  Creation picks, for each row width, the
  * pair-kernel variant (2-6 blocks per SM for 32-bit rows, 2-5 for 64-bit
  * rows), the tasks per resident warp (16,
  * 64, 256) and the kets per chunk (16, 32, 64), in that order, by timing the

@@ -29,7 +29,8 @@ struct HPauli {
     bool anticommutes(const HPauli& o) const { return parity64((x & o.z)) != parity64((z & o.x)); }
 };
 
-// 64×64 bit-matrix transpose in place (row i = word i), by block swaps.
+// 64×64 bit-matrix transpose in place (row i = word i), by recursive block swaps
+// (H. S. Warren, Hacker's Delight, section 7-3).
 inline void transpose64(uint64_t (&a)[64]) {
     uint64_t m = 0x00000000ffffffffull;
     for (int j = 32; j; j >>= 1, m ^= m << j)

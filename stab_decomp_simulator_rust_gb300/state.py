@@ -459,8 +459,10 @@ class BatchPlan:
 def exp_values_multi(states, paulis_per_state, precision: int = PRECISION_FP64,
                      screen: bool = False) -> list[np.ndarray]:
     """⟨P⟩ for many states at once: observables ``paulis_per_state[c]`` on
-    ``states[c]``, every pair sum in one persistent launch (one per row width:
-    ≤ 32 and > 32 qubits).  Returns one array per state, each value as
+    ``states[c]``.  The states are summed together, in at most five sets of
+    launches: pairs from term tables (≤ 32 and > 32 qubits), pairs of reduced
+    terms as quadratic forms (≤ 32 and > 32 qubits left), and amplitudes.
+    Returns one array per state, each value as
     ``states[c].exp_values(paulis_per_state[c], precision)`` gives it.
     screen=True (opt-in): states whose every observable the common-stabilizer
     test (QuantumState.zero_screen) decides get the exact zeros without a pair
